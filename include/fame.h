@@ -104,6 +104,11 @@ FAME_API int fame_mass_apply(fame_mass* m, int mode, const void* x, void* y, int
  * FAME_ERR_CUDA when the timeout was detected (the expected outcome); the fault word is
  * cleared and the context stays usable.  The mass handle's scratch field is overwritten. */
 FAME_API int fame_selftest_bounded_wait(fame_mass* m, unsigned poll_limit);
+/* The same expiry in one kernel, without the report: kernel 0 = pass B (FP32), 1 = pass B of the
+ * mass adjoint, 2 = the Gram-Schmidt tile kernel.  The fault word stays set for the next call
+ * that checks it: fame_ctx_sync, fame_mass_adjoint(_fields), fame_lanczos, fame_osi_eigs,
+ * fame_rayleigh_ritz and the batched solves then fail with FAME_ERR_CUDA. */
+FAME_API int fame_selftest_expired_wait(fame_mass* m, int kernel, unsigned poll_limit);
 
 /* Replaces applyMij_rank1_exact(x,kernelFFT,plan) — exp1/applyMij_rank1_exact.m:1-6
  * with rank1_exact_fft_scatter / rank1_exact_ifft_gather

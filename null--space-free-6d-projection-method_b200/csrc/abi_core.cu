@@ -43,6 +43,7 @@ StreamOrderedAlloc::~StreamOrderedAlloc() {
 constexpr int kMaxDevices = 64;
 static std::atomic<unsigned*> g_fault[kMaxDevices];
 static std::atomic<int> g_sms[kMaxDevices];
+static std::atomic<unsigned> g_faults_seen[kMaxDevices];  // times a check found the fault word set
 static std::mutex g_dev_mu;
 
 static int current_device() {
@@ -174,8 +175,17 @@ int check_fault(fame_ctx* ctx) {
   unsigned v = 0;
   std::memcpy(&v, ctx->pinned, sizeof(unsigned));
   if (v == 0) return FAME_OK;
+  g_faults_seen[ctx->device].fetch_add(1);  // before the word is cleared: see FaultWatch
   FAME_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(unsigned), ctx->stream));
   return fail(FAME_ERR_CUDA, "a bounded device-side wait gave up (bulk copy never completed); results are invalid");
+}
+
+FaultWatch::FaultWatch(fame_ctx* c) : ctx(c), seen(g_faults_seen[c->device].load()) {}
+
+int FaultWatch::check() {
+  FAME_TRY(check_fault(ctx));
+  if (g_faults_seen[ctx->device].load() == seen) return FAME_OK;
+  return fail(FAME_ERR_CUDA, "a bounded device-side wait gave up during this call; results are invalid");
 }
 
 int ctx_workspace(fame_ctx* ctx, size_t bytes, void** out) {

@@ -77,6 +77,20 @@ struct StreamOrderedAlloc {
 int read_back(fame_ctx* ctx, const void* dsrc, void* hdst, size_t bytes);
 // FAME_ERR_CUDA (and clears the word) if a bounded device-side wait gave up on ctx's device
 int check_fault(fame_ctx* ctx);
+// For a call whose own result rests on bounded waits: check() synchronises ctx's stream and
+// fails if any wait of the device gave up since the construction, also where another host
+// thread's check found the device's fault word first and cleared it.
+class FaultWatch {
+  fame_ctx* ctx;
+  unsigned seen;
+
+ public:
+  explicit FaultWatch(fame_ctx* ctx);
+  int check();
+};
+// One block of the Gram-Schmidt tile kernel whose copies never come (lanczos.cu): the kernel
+// sets the fault word and returns.
+int selftest_gram_schmidt_wait(fame_ctx* ctx, unsigned poll_limit);
 // At least `bytes` of device workspace owned by ctx, reused across calls (grown
 // after a stream synchronisation); valid until the next call on the context.
 int ctx_workspace(fame_ctx* ctx, size_t bytes, void** out);

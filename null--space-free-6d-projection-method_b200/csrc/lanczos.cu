@@ -154,7 +154,8 @@ inline size_t fuse_smem(int m) { return (size_t)m * kFuseRows * sizeof(double2);
 __global__ void __launch_bounds__(kFuseThreads) k_cgs_sub_dot(const double2* __restrict__ Q, long long ldq, int m,
                                                               const double2* __restrict__ coef,
                                                               double2* __restrict__ w, long long n,
-                                                              double2* __restrict__ partial, unsigned* fault) {
+                                                              double2* __restrict__ partial, unsigned* fault,
+                                                              unsigned poll_limit = kMbarPollLimit, int arm_only = 0) {
   extern __shared__ __align__(128) double2 qt[];  // [m][kFuseRows]
   __shared__ double2 c[kFuseMaxCols];
   __shared__ double2 half[kFuseRows];
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(kFuseThreads) k_cgs_sub_dot(const double2* __r
     const unsigned bytes = (unsigned)((n - r0 < kFuseRows ? n - r0 : kFuseRows) * sizeof(double2));
     if (lane == 0) mbar_arrive_expect_tx(&bar, bytes * m);
     __syncwarp();
+    if (arm_only) return;  // fault-path self-test: the bytes never come, nothing is in flight
     for (int j = lane; j < m; j += 32) bulk_g2s(qt + j * kFuseRows, Q + ldq * j + r0, bytes, &bar);
   };
   if (threadIdx.x == 0) {
@@ -186,9 +188,12 @@ __global__ void __launch_bounds__(kFuseThreads) k_cgs_sub_dot(const double2* __r
     const int rows = (int)(n - b * kFuseRows < kFuseRows ? n - b * kFuseRows : kFuseRows);
     double2 v = make_double2(0.0, 0.0);
     if (h == 0 && r < rows) v = w[row];
-    const bool landed = mbar_wait(&bar, phase);
+    const bool landed = mbar_wait(&bar, phase, poll_limit);
     if (!__syncthreads_and(landed)) {  // bounded wait, agreed on by the whole CTA
-      if (fault && threadIdx.x == 0) atomicOr(fault, 1u);
+      if (threadIdx.x == 0) {
+        mbar_wait(&bar, phase, poll_limit);  // copies in flight still land in this CTA's shared memory
+        if (fault) atomicOr(fault, 1u);
+      }
       return;
     }
     {  // columns h, h + 2, ... of this row in two partial sums
@@ -544,11 +549,25 @@ void lanczos_ws_release(void** ws) {
 
 void lanczos_ws_free(fame_krinv* K) { lanczos_ws_release(&K->lanczos_ws); }
 
+int selftest_gram_schmidt_wait(fame_ctx* ctx, unsigned poll_limit) {
+  constexpr int m = 2;
+  void* buf = nullptr;  // Q (m columns), w, coefficients, partial sums
+  const size_t elems = (size_t)(m + 1) * kFuseRows + 2 * m;
+  FAME_TRY(dalloc(&buf, elems * sizeof(double2)));
+  double2* Q = static_cast<double2*>(buf);
+  double2 *w = Q + m * kFuseRows, *coef = w + kFuseRows, *partial = coef + m;
+  cudaMemsetAsync(buf, 0, elems * sizeof(double2), ctx->stream);
+  k_cgs_sub_dot<<<1, kFuseThreads, fuse_smem(m), ctx->stream>>>(Q, kFuseRows, m, coef, w, kFuseRows, partial,
+                                                                fault_word(), poll_limit, 1);
+  ::fame::count_launch();
+  const cudaError_t e = cudaGetLastError();
+  dfree(buf);
+  return e == cudaSuccess ? FAME_OK : fail(FAME_ERR_CUDA, "self-test launch");
+}
+
 // Restarted Lanczos for the largest (algebraic) eigenvalues of a Hermitian operator.
-int lanczos_run(const LanczosOperator& op, int nev, double tol, int maxiter, int p, const void* v0, double* theta,
-                void* Y, fame_lanczos_info* info) {
-  if (!op.ctx || !op.apply || !op.ws || !v0 || !theta || nev < 1 || p < nev + 1 || p > kMaxCols || maxiter < 1)
-    return fail(FAME_ERR_INVALID, "Lanczos arguments (need 1 <= nev < p <= 256)");
+static int lanczos_solve(const LanczosOperator& op, int nev, double tol, int maxiter, int p, const void* v0,
+                         double* theta, void* Y, fame_lanczos_info* info) {
   fame_ctx* ctx = op.ctx;
   cudaStream_t s = ctx->stream;
   const long long n = op.n;
@@ -691,8 +710,18 @@ int lanczos_run(const LanczosOperator& op, int nev, double tol, int maxiter, int
     info->nconv = nconv;
     info->maxWantedResidual = maxres;
   }
-  FAME_CUDA_TRY(cudaStreamSynchronize(s));
   return FAME_OK;
+}
+
+int lanczos_run(const LanczosOperator& op, int nev, double tol, int maxiter, int p, const void* v0, double* theta,
+                void* Y, fame_lanczos_info* info) {
+  if (!op.ctx || !op.apply || !op.ws || !v0 || !theta || nev < 1 || p < nev + 1 || p > kMaxCols || maxiter < 1)
+    return fail(FAME_ERR_INVALID, "Lanczos arguments (need 1 <= nev < p <= 256)");
+  // a wait that gave up leaves finite but wrong coefficients behind: it outranks any other outcome
+  FaultWatch watch(op.ctx);
+  const int st = lanczos_solve(op, nev, tol, maxiter, p, v0, theta, Y, info);
+  FAME_TRY(watch.check());
+  return st;
 }
 
 }  // namespace fame

@@ -140,9 +140,9 @@ __global__ void __launch_bounds__(32 * kAdjWarps) k_adjoint_gemm(const double* _
 
 // densities of `modes` consecutive modes (x: 3 NF each) through work (3 modes fields)
 template <int n>
-int adjoint_density_n(const double2* x, double2* work, double* dens, int modes, long long NF, cudaStream_t st) {
+int launch_density(const double2* work, double* dens, int modes, long long NF, cudaStream_t st,
+                   unsigned poll_limit = kMbarPollLimit, int arm_only = 0) {
   using G = PassBGeom<n, double>;
-  FAME_TRY((passA_cols_n<n, double>(x, 3 * modes, work, NF, st)));
   constexpr size_t smem = 2 * (size_t)G::stage * sizeof(double2) + 2 * sizeof(uint64_t);
   static int attr = ensure_smem(k_passB_density<n>, smem);
   if (attr != FAME_OK) return attr;
@@ -152,10 +152,15 @@ int adjoint_density_n(const double2* x, double2* work, double* dens, int modes, 
     return b < 1 ? 1 : b;
   }();
   const int grid = std::min((G::n3 / G::TT) * modes, per_sm * num_sms());
-  k_passB_density<n><<<grid, G::threads, smem, st>>>(work, dens, modes, NF, fault_word());
+  k_passB_density<n><<<grid, G::threads, smem, st>>>(work, dens, modes, NF, fault_word(), poll_limit, arm_only);
   ::fame::count_launch();
   FAME_CUDA_TRY(cudaGetLastError());
   return FAME_OK;
+}
+template <int n>
+int adjoint_density_n(const double2* x, double2* work, double* dens, int modes, long long NF, cudaStream_t st) {
+  FAME_TRY((passA_cols_n<n, double>(x, 3 * modes, work, NF, st)));
+  return launch_density<n>(work, dens, modes, NF, st);
 }
 
 int check_N(int N) {
@@ -308,9 +313,29 @@ int fame_mass_destroy(fame_mass* m) {
 
 int fame_selftest_bounded_wait(fame_mass* m, unsigned poll_limit) {
   if (!m) return fail(FAME_ERR_INVALID, "fame_selftest_bounded_wait: mass is NULL");
+  FAME_TRY(check_fault(m->ctx));  // start from a clear fault word
+  FAME_TRY(fame_selftest_expired_wait(m, 0, poll_limit));
+  return check_fault(m->ctx);  // FAME_ERR_CUDA: the timeout was detected and reported
+}
+
+int fame_selftest_expired_wait(fame_mass* m, int kernel, unsigned poll_limit) {
+  if (!m || kernel < 0 || kernel > 2) return fail(FAME_ERR_INVALID, "fame_selftest_expired_wait arguments");
   if (poll_limit < 1 || poll_limit > (1u << 20)) return fail(FAME_ERR_INVALID, "poll_limit must be in [1, 2^20]");
   fame_ctx* ctx = m->ctx;
-  FAME_TRY(check_fault(ctx));  // start from a clear fault word
+  if (kernel == 2) return selftest_gram_schmidt_wait(ctx, poll_limit);
+  if (kernel == 1) {  // no CTA gets as far as the densities: the scratch field stands in for them
+    const double2* w64 = static_cast<const double2*>(m->work);
+    double* d = static_cast<double*>(m->work);
+    switch (m->n) {
+      case 2: return launch_density<2>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+      case 4: return launch_density<4>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+      case 6: return launch_density<6>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+      case 8: return launch_density<8>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+      case 10: return launch_density<10>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+      case 12: return launch_density<12>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+      default: return launch_density<14>(w64, d, 1, m->NF, ctx->stream, poll_limit, 1);
+    }
+  }
   // one FP32 field in the handle's scratch (8 NF bytes of its 16 NF); every stage barrier
   // expects bytes that no copy delivers, so each CTA's first wait runs out and returns
   float2* w = reinterpret_cast<float2*>(m->work);
@@ -327,7 +352,7 @@ int fame_selftest_bounded_wait(fame_mass* m, unsigned poll_limit) {
   }
   FAME_TRY(s);
   FAME_CUDA_TRY(cudaGetLastError());
-  return check_fault(ctx);  // FAME_ERR_CUDA: the timeout was detected and reported
+  return FAME_OK;
 }
 
 int fame_mass_apply(fame_mass* m, int mode, const void* x, void* y, int nrhs, int prec) {
@@ -371,6 +396,7 @@ int fame_mass_adjoint_fields(fame_mass* m, const void* X, int nmodes, const doub
   cv = Carve{};
   cv.base = static_cast<char*>(ws);
   carve(cv);
+  FaultWatch watch(m->ctx);
   int s = cudaMemsetAsync(counter, 0, sizeof(unsigned), st) == cudaSuccess ? FAME_OK : fail(FAME_ERR_CUDA, "adjoint");
   for (int j0 = 0; j0 < nmodes && s == FAME_OK; j0 += 16) {
     const int jn = std::min(16, nmodes - j0);
@@ -397,9 +423,10 @@ int fame_mass_adjoint_fields(fame_mass* m, const void* X, int nmodes, const doub
     if (cudaGetLastError() != cudaSuccess) s = fail(FAME_ERR_CUDA, "adjoint launch");
   }
   std::vector<double> h((size_t)groups * 128);
-  if (s == FAME_OK && (cudaMemcpyAsync(h.data(), res, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                       cudaStreamSynchronize(st) != cudaSuccess))
+  if (s == FAME_OK &&
+      cudaMemcpyAsync(h.data(), res, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     s = fail(FAME_ERR_CUDA, "adjoint");
+  if (s == FAME_OK) s = watch.check();  // synchronises; a copy that never came leaves densities unwritten
   dfree(ws);
   FAME_TRY(s);
   for (int j = 0; j < nmodes; ++j)

@@ -110,7 +110,12 @@ __global__ void __launch_bounds__(PassBGeom<n, T>::maxThreads, PassBGeom<n, T>::
     const int s = i & 1;
     const bool landed = mbar_wait(&bar[s], (unsigned)((i >> 1) & 1), poll_limit);
     if (!__syncthreads_and(landed)) {  // bounded wait, agreed on by the whole CTA
-      if (fault && tid == 0) atomicOr(fault, 1u);
+      if (tid == 0) {
+        // copies in flight still land in this CTA's shared memory: wait for them (bounded) before it exits
+        mbar_wait(&bar[s], (unsigned)((i >> 1) & 1), poll_limit);
+        if (u + 1 < u1) mbar_wait(&bar[s ^ 1], (unsigned)(((i + 1) >> 1) & 1), poll_limit);
+        if (fault) atomicOr(fault, 1u);
+      }
       return;
     }
     C<T>* S = stg + s * G::stage;
@@ -179,7 +184,8 @@ __global__ void __launch_bounds__(PassBGeom<n, T>::maxThreads, PassBGeom<n, T>::
 // the three fields of a pair accumulate in the registers of the last axis' lines.
 template <int n>
 __global__ void __launch_bounds__((PassBGeom<n, double>::threads), n >= 10 && n < 14 ? 2 : 0)
-k_passB_density(const double2* __restrict__ work, double* __restrict__ dens, int modes, long long NF, unsigned* fault) {
+k_passB_density(const double2* __restrict__ work, double* __restrict__ dens, int modes, long long NF, unsigned* fault,
+                unsigned poll_limit = kMbarPollLimit, int arm_only = 0) {
   using G = PassBGeom<n, double>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double2* stg = reinterpret_cast<double2*>(smem_raw);
@@ -191,6 +197,7 @@ k_passB_density(const double2* __restrict__ work, double* __restrict__ dens, int
   auto issue = [&](int i) {
     const int p = p0 + i / 3, k = p / modes, md = p - k * modes, s = i & 1;
     mbar_arrive_expect_tx(&bar[s], n * G::plane_bytes);
+    if (arm_only) return;  // fault-path self-test, as in k_passB
     const double2* src = work + (3LL * md + i % 3) * NF + (long long)k * G::tile;
 #pragma unroll 1
     for (int q = 0; q < n; ++q)
@@ -210,9 +217,13 @@ k_passB_density(const double2* __restrict__ work, double* __restrict__ dens, int
 #pragma unroll 1
   for (int i = 0; i < units; ++i) {
     const int s = i & 1, f = i % 3;
-    const bool landed = mbar_wait(&bar[s], (unsigned)((i >> 1) & 1));
+    const bool landed = mbar_wait(&bar[s], (unsigned)((i >> 1) & 1), poll_limit);
     if (!__syncthreads_and(landed)) {  // bounded wait, agreed on by the whole CTA
-      if (fault && tid == 0) atomicOr(fault, 1u);
+      if (tid == 0) {  // copies in flight land first, as in k_passB
+        mbar_wait(&bar[s], (unsigned)((i >> 1) & 1), poll_limit);
+        if (i + 1 < units) mbar_wait(&bar[s ^ 1], (unsigned)(((i + 1) >> 1) & 1), poll_limit);
+        if (fault) atomicOr(fault, 1u);
+      }
       return;
     }
     double2* S = stg + s * G::stage;

@@ -80,6 +80,7 @@ SIGNATURES = {
     "fame_mass_destroy": [P],
     "fame_mass_apply": [P, I, P, P, I, I],
     "fame_selftest_bounded_wait": [P, C.c_uint],
+    "fame_selftest_expired_wait": [P, I, C.c_uint],
     "fame_applyMij_rank1_exact": [P, P, P, LL, P, P, I],
     "fame_rank1_exact_fft_scatter": [P, P, I, P, LL, LL, P],
     "fame_rank1_exact_ifft_gather": [P, P, I, P, LL, LL, P],
