@@ -13,7 +13,9 @@
  *    [0..N-1, -N..-1] per axis; 2NF/3NF vectors are component-stacked.
  *  - Buffers are caller-owned; handles own their workspace.  A handle is used
  *    from one host thread at a time.  Work is ordered on the context's stream
- *    (fame_ctx_set_stream); calls that return host values synchronise it.
+ *    (fame_ctx_set_stream); calls that return host values synchronise it.  A handle's
+ *    set-up is work of the stream that was current when it was made: a caller that
+ *    changes the stream orders the new one behind it, as with any other device data.
  *  - The reference functions each entry point replaces are cited as
  *    file:line inside the reference project (MATLAB).
  */

@@ -801,6 +801,12 @@ int recover_exact(fame_basis* b, fame_mass* m, const double2* Y, int k, double t
   fame_ctx* ctx = b->ctx;
   cudaStream_t s = ctx->stream;
   const long long NF = b->NF;
+  for (int j = 0; j < k; ++j) relres[j] = -1.0;
+  // the range first: it orders the chains behind the mass handle's set-up on whatever stream that
+  // ran, and a material they do not invert costs nothing here
+  MaterialRange r{};
+  FAME_TRY(read_range(ctx, m, &r));
+  if (!exact_inverse_ok(r, tol)) return FAME_OK;
   double2* work;
   double *partials, *out;
   unsigned* counter;
@@ -828,20 +834,16 @@ int recover_exact(fame_basis* b, fame_mass* m, const double2* Y, int k, double t
       st = run_chain<double, 3>(b->n, ProScaleRec{Xj, oj, NF}, EpiMassRec{vy, MXj, oj, partials, counter}, work,
                                 m->Et64, NF, s);
   }
-  MaterialRange r{};
   std::vector<double> h((size_t)k * 4, 0.0);
-  if (st == FAME_OK) {
-    if (cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess)
-      st = fail(FAME_ERR_CUDA, "recovery");
-    if (st == FAME_OK) st = read_range(ctx, m, &r);
-  }
+  if (st == FAME_OK &&
+      (cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+       cudaStreamSynchronize(s) != cudaSuccess))
+    st = fail(FAME_ERR_CUDA, "recovery");
   dfree(ws);
   FAME_TRY(st);
-  const bool invertible = exact_inverse_ok(r, tol);
   for (int j = 0; j < k; ++j) {
     const double xb = h[4 * j], bb = h[4 * j + 1], rr = h[4 * j + 2];
-    relres[j] = -1.0;
-    if (!invertible || !(xb > 0.0) || !std::isfinite(xb) || !(rr >= 0.0)) continue;
+    if (!(xb > 0.0) || !std::isfinite(xb) || !(rr >= 0.0)) continue;
     const double rel = std::sqrt(rr * xb / bb);
     if (rel <= tol) relres[j] = rel;
   }
