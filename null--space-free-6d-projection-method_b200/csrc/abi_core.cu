@@ -46,7 +46,7 @@ static std::atomic<int> g_sms[kMaxDevices];
 static std::atomic<unsigned> g_faults_seen[kMaxDevices];  // times a check found the fault word set
 static std::mutex g_dev_mu;
 
-static int current_device() {
+int current_device() {
   int d = 0;
   if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= kMaxDevices) return -1;
   return d;

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <string>
 #include "../../include/fame.h"
+#include "device_once.h"
 
 namespace fame {
 
@@ -67,6 +68,16 @@ void count_launch(long long n = 1);
 // before a context exists on the current device) and SM count of the current device.
 unsigned* fault_word();
 int num_sms();
+int current_device();  // -1 if the runtime has none or the library no state for it
+// Dynamic shared-memory limit of a kernel for launches with up to `bytes`: an attribute that every
+// device holds for itself, so `once` (a static beside the launch) remembers it per device.
+template <typename K> int ensure_smem(K kernel, size_t bytes, DeviceOnce& once) {
+  if (bytes <= 48 * 1024) return FAME_OK;
+  return once(current_device(), [&] {
+    FAME_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return FAME_OK;
+  });
+}
 
 // --------------------------------------------------------------- reductions
 // Sum of K accumulators.  Each block reduces its threads' values, writes

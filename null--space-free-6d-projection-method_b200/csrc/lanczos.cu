@@ -486,9 +486,8 @@ struct LanczosWs {
   // (k_cgs_sub_dot, m <= 64), so two passes read Q three times instead of four.
   int cgs(int m, int passes) {
     cudaStream_t s = ctx->stream;
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_cgs_sub_dot, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fuse_smem(kFuseMaxCols));
-    FAME_CUDA_TRY(attr);
+    static DeviceOnce once;
+    FAME_TRY(ensure_smem(k_cgs_sub_dot, fuse_smem(kFuseMaxCols), once));
     gemv_h(m);
     k_gemv_h_reduce<<<m, 256, 0, s>>>(partial, nblk, m, coef, scal, 1);
     ::fame::count_launch();

@@ -144,8 +144,8 @@ int launch_density(const double2* work, double* dens, int modes, long long NF, c
                    unsigned poll_limit = kMbarPollLimit, int arm_only = 0) {
   using G = PassBGeom<n, double>;
   constexpr size_t smem = 2 * (size_t)G::stage * sizeof(double2) + 2 * sizeof(uint64_t);
-  static int attr = ensure_smem(k_passB_density<n>, smem);
-  if (attr != FAME_OK) return attr;
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_passB_density<n>, smem, once));
   static int per_sm = [] {
     int b = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_passB_density<n>, G::threads, smem) != cudaSuccess) b = 1;

@@ -7,13 +7,6 @@ namespace fame {
 
 inline int round32(int x) { return (x + 31) / 32 * 32; }
 
-// Set the dynamic shared-memory limit of a kernel once per process.
-template <typename K> int ensure_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return FAME_OK;
-  FAME_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return FAME_OK;
-}
-
 // Pass B over nfields tile-major fields with the tiled material Et (E/NF in the
 // layout of k_tile_E for this n and T): a persistent grid of (resident CTAs per
 // SM) x SMs, each CTA owning a contiguous range of (tile, field) units.
@@ -23,8 +16,8 @@ int launch_passB(C<T>* work, int nfields, const TE* Et, long long NF, cudaStream
                  unsigned poll_limit = kMbarPollLimit, int arm_only = 0) {
   using G = PassBGeom<n, T>;
   constexpr size_t smem = G::template smem_bytes<TE>();
-  static int attr = ensure_smem(k_passB<n, T, TE>, smem);
-  if (attr != FAME_OK) return attr;
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_passB<n, T, TE>, smem, once));
   static int per_sm = [] {
     int b = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_passB<n, T, TE>, G::threads, smem) != cudaSuccess) b = 1;
@@ -48,8 +41,8 @@ int launch_passA(const Pro& pro, C<T>* work, long long NF, cudaStream_t st, Gate
   using Q = Cube<n, T>;
   constexpr int G = PassACols<n, T>::value;
   const size_t smem = (size_t)G * F * Q::size * sizeof(C<T>);
-  static int attr = ensure_smem(k_passA<n, T, F, G, Pro>, smem);
-  if (attr != FAME_OK) return attr;
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_passA<n, T, F, G, Pro>, smem, once));
   const int threads = pass_threads<n, T, F>(G);
   k_passA<n, T, F, G, Pro><<<Q::n3 / G, threads, smem, st>>>(pro, work, NF, gate);
   ::fame::count_launch();
@@ -61,8 +54,8 @@ int launch_passC(const Epi& epi, const C<T>* work, long long NF, cudaStream_t st
   using Q = Cube<n, T>;
   constexpr int G = PassACols<n, T>::value;
   const size_t smem = (size_t)G * F * Q::size * sizeof(C<T>);
-  static int attr = ensure_smem(k_passC<n, T, F, G, Epi>, smem);
-  if (attr != FAME_OK) return attr;
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_passC<n, T, F, G, Epi>, smem, once));
   const int threads = pass_threads<n, T, F>(G);
   k_passC<n, T, F, G, Epi><<<Q::n3 / G, threads, smem, st>>>(epi, work, NF, gate);
   ::fame::count_launch();
@@ -114,10 +107,10 @@ int chain_lin_g(const Pro& pro, const Epi& epi, C<T>* work, const TE* Et, long l
   using Q = Cube<n, T>;
   const size_t smem = (size_t)G * Q::size * sizeof(C<T>);
   const int threads = round32(G * Q::n2);
-  static int attrA = ensure_smem(k_passA_lin<n, T, F, G, Pro>, smem);
-  static int attrC = ensure_smem(k_passC_lin<n, T, F, G, Epi>, smem);
-  if (attrA != FAME_OK) return attrA;
-  if (attrC != FAME_OK) return attrC;
+  static DeviceOnce onceA;
+  FAME_TRY(ensure_smem(k_passA_lin<n, T, F, G, Pro>, smem, onceA));
+  static DeviceOnce onceC;
+  FAME_TRY(ensure_smem(k_passC_lin<n, T, F, G, Epi>, smem, onceC));
   k_passA_lin<n, T, F, G, Pro><<<Q::n3 / G, threads, smem, st>>>(pro, work, NF, gate);
   ::fame::count_launch();
   FAME_TRY((launch_passB<n, T, TE>(work, F, Et, NF, st, gate)));
@@ -134,10 +127,10 @@ int chain_par(const Pro& pro, const Epi& epi, C<T>* work, const TE* Et, long lon
   constexpr int G = 1;
   const size_t smA = (size_t)G * (F + 1) * Q::size * sizeof(C<T>), smC = (size_t)G * F * Q::size * sizeof(C<T>);
   const int threads = round32(F * G * Q::n2);
-  static int attrA = ensure_smem(k_passA_par<n, T, F, G, Pro>, smA);
-  static int attrC = ensure_smem(k_passC_par<n, T, F, G, Epi>, smC);
-  if (attrA != FAME_OK) return attrA;
-  if (attrC != FAME_OK) return attrC;
+  static DeviceOnce onceA;
+  FAME_TRY(ensure_smem(k_passA_par<n, T, F, G, Pro>, smA, onceA));
+  static DeviceOnce onceC;
+  FAME_TRY(ensure_smem(k_passC_par<n, T, F, G, Epi>, smC, onceC));
   k_passA_par<n, T, F, G, Pro><<<Q::n3 / G, threads, smA, st>>>(pro, work, NF, gate);
   FAME_TRY((launch_passB<n, T, TE>(work, F, Et, NF, st, gate)));
   k_passC_par<n, T, F, G, Epi><<<Q::n3 / G, threads, smC, st>>>(epi, work, NF, gate);
@@ -240,8 +233,8 @@ template <int n, typename T> int passA_cols_n(const C<T>* x, int nvec, C<T>* wor
   using Q = Cube<n, T>;
   constexpr int G = LinCols<n, T>::value;
   const size_t smem = (size_t)G * Q::size * sizeof(C<T>);
-  static int attr = ensure_smem(k_passA_lin<n, T, 1, G, ProCol<T>>, smem);
-  if (attr != FAME_OK) return attr;
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_passA_lin<n, T, 1, G, ProCol<T>>, smem, once));
   k_passA_lin<n, T, 1, G, ProCol<T>>
       <<<dim3(Q::n3 / G, nvec), round32(G * Q::n2), smem, st>>>(ProCol<T>{x, NF}, work, NF, Gate{nullptr});
   ::fame::count_launch();
@@ -257,8 +250,8 @@ int mass_cols_n(const C<T>* x, C<T>* y, int nvec, C<T>* work, const TE* Et, long
   const size_t smem = (size_t)G * Q::size * sizeof(C<T>);
   const int threads = round32(G * Q::n2);
   const dim3 grid(Q::n3 / G, nvec);
-  static int attrC = ensure_smem(k_passC_lin<n, T, 1, G, EpiCol<T>>, smem);
-  if (attrC != FAME_OK) return attrC;
+  static DeviceOnce onceC;
+  FAME_TRY(ensure_smem(k_passC_lin<n, T, 1, G, EpiCol<T>>, smem, onceC));
   FAME_TRY((passA_cols_n<n, T>(x, nvec, work, NF, st)));
   FAME_TRY((launch_passB<n, T, TE>(work, nvec, Et, NF, st, Gate{nullptr})));
   k_passC_lin<n, T, 1, G, EpiCol<T>><<<grid, threads, smem, st>>>(EpiCol<T>{y, NF}, work, NF, Gate{nullptr});

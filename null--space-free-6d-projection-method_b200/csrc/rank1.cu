@@ -143,11 +143,8 @@ int launch_pass(int R, const double2* in, double2* out, long long M, long long N
     const long long T = M / RR;
     if (Ns == 1) {
       constexpr size_t smem = (size_t)kFirstThreads * RR * sizeof(double2);
-      static int attr = cudaFuncSetAttribute(k_stockham_first<RR, SIGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem) == cudaSuccess
-                            ? FAME_OK
-                            : fail(FAME_ERR_CUDA, "rank-1 FFT: shared-memory limit");
-      FAME_TRY(attr);
+      static DeviceOnce once;
+      FAME_TRY(ensure_smem(k_stockham_first<RR, SIGN>, smem, once));
       const int blocks = (int)std::min<long long>((T + kFirstThreads - 1) / kFirstThreads, (long long)num_sms() * 8);
       k_stockham_first<RR, SIGN><<<blocks, kFirstThreads, smem, s>>>(in, out, M);
     } else {

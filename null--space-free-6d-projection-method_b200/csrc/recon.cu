@@ -255,11 +255,8 @@ __global__ void __launch_bounds__(kGThreads, 3) k_zgemm_mma(GemmArgs g) {
 }
 
 int zgemm(const GemmArgs& g, int batch, cudaStream_t s) {
-  static int attr = cudaFuncSetAttribute(k_zgemm_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGSmem) ==
-                            cudaSuccess
-                        ? FAME_OK
-                        : FAME_ERR_CUDA;
-  if (attr != FAME_OK) return fail(attr, "zgemm: shared-memory limit");
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_zgemm_mma, kGSmem, once));
   if (g.K > kGMaxK) return fail(FAME_ERR_UNSUPPORTED, "zgemm: contraction too long");
   auto tiles = [](int d) { return ((d + 7) / 8 + kGBlk - 1) / kGBlk; };
   dim3 grid(tiles(g.M), tiles(g.N), batch);
@@ -544,11 +541,8 @@ int launch_moments_mma(const double2* c, const double* Q, long long NF, const do
   constexpr size_t smem = (size_t)(16 * WM + 128 / WM * NT) * kMmaPitch * sizeof(double) +
                           6 * (kMaxP + 1) * kMmaModes * sizeof(double) + 128 / WM * NT * sizeof(int);
   static_assert(smem <= 227 * 1024, "operand stage");
-  static int attr = cudaFuncSetAttribute(k_taylor_moments_mma<NT, WM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem) == cudaSuccess
-                        ? FAME_OK
-                        : FAME_ERR_CUDA;
-  if (attr != FAME_OK) return fail(attr, "Taylor moments: shared-memory limit");
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_taylor_moments_mma<NT, WM>, smem, once));
   k_taylor_moments_mma<NT, WM><<<dim3(nslices, (nB + 8 * WM - 1) / (8 * WM), groups), 512, smem, s>>>(
       c, Q, NF, centers, runs, L, nB, per_slice, partial);
   ::fame::count_launch();

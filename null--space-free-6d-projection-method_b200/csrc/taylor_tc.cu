@@ -441,13 +441,8 @@ int taylor_moments_tc(const TaylorTcPlan& pl, cudaStream_t s, const double2* c, 
   if (grid.ax && (grid.m1 < 1 || grid.m2 < 1 || grid.m3 < 1 || grid.m1 * grid.m2 * grid.m3 != nB ||
                   grid.m1 + grid.m2 + grid.m3 > kMaxAxis))
     return fail(FAME_ERR_INVALID, "tensor-core Taylor moments: bad center grid");
-  static int attr = [] {
-    return cudaFuncSetAttribute(k_taylor_moments_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
-                   cudaSuccess
-               ? FAME_OK
-               : FAME_ERR_CUDA;
-  }();
-  if (attr != FAME_OK) return fail(attr, "tensor-core Taylor moments: shared-memory limit");
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_taylor_moments_tc, 227 * 1024, once));
   TcArgs a{Q, c, NF, centers, nB, alistPacked, col, L, p, pl.Npad, pl.Nc, pl.Csep, pl.stages, pl.Kc, out,
            grid.ax, grid.m1, grid.m2, grid.m3};
   dim3 g3((unsigned)pl.nslices, (unsigned)pl.ntiles, (unsigned)pl.nsplit);

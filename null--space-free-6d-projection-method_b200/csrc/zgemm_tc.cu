@@ -433,13 +433,8 @@ int launch_zgemm(ZgArgs g, int batch, cudaStream_t s) {
     return fail(FAME_ERR_INVALID, "zgemm_3xtf32: panels must be 1024-byte aligned");
   g.Nt = z_nt(g.N);
   g.S = zstages(g.Nt);
-  static int attr = [] {
-    return cudaFuncSetAttribute(k_zgemm_3xtf32<OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
-                   cudaSuccess
-               ? FAME_OK
-               : FAME_ERR_CUDA;
-  }();
-  if (attr != FAME_OK) return fail(attr, "zgemm_3xtf32: shared-memory limit");
+  static DeviceOnce once;
+  FAME_TRY(ensure_smem(k_zgemm_3xtf32<OUT>, 227 * 1024, once));
   const long long gy = ((long long)g.N + g.Nt - 1) / g.Nt;
   if (gy > 65535 || batch > 65535) return fail(FAME_ERR_UNSUPPORTED, "zgemm_3xtf32: grid too large");
   g.tilesM = (g.M + kZM - 1) / kZM;
