@@ -133,10 +133,10 @@ __global__ void k_build_basis(BasisArgs a) {
   }
 }
 
-// dst = src + 0i
-__global__ void k_widen(const double* src, double2* dst, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = make_double2(src[i], 0.0);
+// dst (interleaved re, im; 8-byte aligned) = src + 0i
+__global__ void k_widen(const double* src, double* dst, long long n) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 2 * n; t += (long long)gridDim.x * blockDim.x)
+    dst[t] = t & 1 ? 0.0 : src[t >> 1];
 }
 
 // ------------------------------------------------------------ raw maps
@@ -471,11 +471,27 @@ int fame_basis_get(fame_basis* b, int which, void* dst) {
   else return fail(FAME_ERR_INVALID, "unknown basis diagonal");
   if (which >= 9) {
     FAME_CUDA_TRY(cudaMemcpyAsync(dst, src, b->NF * sizeof(double), cudaMemcpyDeviceToDevice, b->ctx->stream));
-  } else {  // the complex diagonals are held by their (only nonzero) real parts
-    k_widen<<<ew_blocks(b->NF), 256, 0, b->ctx->stream>>>(src, (double2*)dst, b->NF);
-    ::fame::count_launch();
-    FAME_CUDA_TRY(cudaGetLastError());
+    return FAME_OK;
   }
+  // the complex diagonals are held by their (only nonzero) real parts: widened into dst where a
+  // kernel of this device can store, and through a buffer that is then copied, as the real
+  // diagonals are, where it cannot (another GPU's memory, the host's, odd addresses)
+  cudaStream_t s = b->ctx->stream;
+  cudaPointerAttributes at{};
+  const bool direct = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+                      at.device == b->ctx->device && reinterpret_cast<uintptr_t>(dst) % sizeof(double) == 0;
+  cudaGetLastError();
+  void* out = dst;
+  if (!direct) FAME_TRY(dalloc(&out, b->NF * sizeof(double2)));
+  k_widen<<<ew_blocks(b->NF), 256, 0, s>>>(src, static_cast<double*>(out), b->NF);
+  ::fame::count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (!direct) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dst, out, b->NF * sizeof(double2), cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    dfree(out);
+  }
+  FAME_CUDA_TRY(e);
   return FAME_OK;
 }
 
