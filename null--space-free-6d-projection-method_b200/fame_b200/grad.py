@@ -27,8 +27,10 @@ def mass_adjoint(mass: MassBackend, X, dEps):
     Xc = X.t().contiguous()
     k = Xc.shape[0]
     G = [g.reshape(-1).contiguous() for g in dEps]
-    if any(g.dtype != torch.float64 or g.numel() != mass.NF for g in G):
-        raise ValueError("dEps must be float64 fields with NF entries")
+    if any(g.dtype != torch.float64 or g.is_neg() for g in G):
+        G = list(torch.stack(G))  # fields of several types become the common one
+    if any(g.dtype != torch.float64 or g.numel() != mass.NF or not g.is_cuda for g in G):
+        raise ValueError("dEps must be float64 device fields with NF entries")
     out = (C.c_double * (k * len(G)))()
     mass.ctx.bind()
     call("fame_mass_adjoint_fields", mass.h, _ptr(Xc), k, (C.c_void_p * len(G))(*[g.data_ptr() for g in G]), len(G),
