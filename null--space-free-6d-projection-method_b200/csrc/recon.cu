@@ -259,10 +259,17 @@ int zgemm(const GemmArgs& g, int batch, cudaStream_t s) {
   FAME_TRY(ensure_smem(k_zgemm_mma, kGSmem, once));
   if (g.K > kGMaxK) return fail(FAME_ERR_UNSUPPORTED, "zgemm: contraction too long");
   auto tiles = [](int d) { return ((d + 7) / 8 + kGBlk - 1) / kGBlk; };
-  dim3 grid(tiles(g.M), tiles(g.N), batch);
-  if (grid.y > 65535) return fail(FAME_ERR_UNSUPPORTED, "zgemm: N too large");
-  k_zgemm_mma<<<grid, kGThreads, kGSmem, s>>>(g);
-  ::fame::count_launch();
+  // 65535 tiles of columns per launch; only the last two GEMMs of long axes have more (a gathered
+  // B has (2N)^4 columns)
+  constexpr int kMaxN = 65535 * kGTile;
+  for (long long n0 = 0; n0 < g.N; n0 += kMaxN) {
+    GemmArgs part = g;
+    part.N = (int)std::min<long long>(kMaxN, g.N - n0);
+    part.B += n0 * g.sbn;
+    part.C += n0 * g.scn;
+    k_zgemm_mma<<<dim3(tiles(part.M), tiles(part.N), batch), kGThreads, kGSmem, s>>>(part);
+    ::fame::count_launch();
+  }
   FAME_CUDA_TRY(cudaGetLastError());
   return FAME_OK;
 }

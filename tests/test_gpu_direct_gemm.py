@@ -61,3 +61,31 @@ def test_direct_grid_tensor_core_chain(cuda_device, N, sizes, ncomp):
         u = F.reconstruct_fields_direct_grid(c, sg, axes, tensor_cores=True)
         for comp in range(ncomp):
             assert torch.linalg.norm(u[comp] - ref[comp]) < 4e-6 * torch.linalg.norm(ref[comp])
+
+
+@pytest.mark.parametrize("axis", [1, 2])
+def test_direct_grid_axis_longer_than_one_launch(cuda_device, axis):
+    """y or z axes with more column tiles (48 points) than one launch's 65535: the points at both
+    ends of each launch against the 64 terms in NumPy, relative 1e-12 (phases of up to 5 radians)."""
+    import torch
+    import fame_b200 as F
+    N, n, edge = 1, 2, 65535 * 48
+    P = np.asarray(F.configs.P_GOLDEN)
+    sg = F.build_q_system(F.MassBackend(torch.as_tensor(O.material_smooth_exp(N), device=cuda_device), N), P,
+                          F.configs.Q_PHYS)
+    rng = np.random.default_rng(axis)
+    c = rng.standard_normal(64) + 1j * rng.standard_normal(64)
+    axes = [rng.uniform(-1, 1, size=edge + 100 if d == axis else 1) for d in range(3)]
+    u = F.reconstruct_field_direct_grid(torch.as_tensor(c, device=cuda_device), sg,
+                                        [torch.as_tensor(a, device=cuda_device) for a in axes]).cpu().numpy()
+    xi = np.array([0.0, -1.0])
+    j = np.arange(64)
+    k = np.asarray(sg.kLift)
+    q = np.zeros((3, 64))
+    for ell in range(6):
+        q += P[ell][:, None] * (xi[(j >> ell) & 1] + k[ell])[None, :]
+    at = np.concatenate([np.arange(50), np.arange(edge - 50, edge + 100)])
+    for i in at:
+        r = np.array([axes[d][i if d == axis else 0] for d in range(3)])
+        ref = np.sum(c * np.exp(1j * (r @ q)))
+        assert abs(u[i] - ref) < 1e-12 * np.linalg.norm(c) * 8
