@@ -17,6 +17,7 @@
 #include <vector>
 #include "internal.cuh"
 #include "dmma.cuh"
+#include "moment_slices.h"
 #include "trig.cuh"
 
 namespace fame {
@@ -557,16 +558,11 @@ int launch_moments_mma(const double2* c, const double* Q, long long NF, const do
   return FAME_OK;
 }
 
-// Slices of the modes: whole waves of one CTA per SM over (slice, center block, column group),
-// at most kMmaSlice modes and at least four stages each.
+// Slices of the modes: whole waves of one CTA per SM over (slice, center block, column group).
 static void moments_mma_slices(long long NF, int nB, int L, int* nslices, long long* per_slice) {
   const int wm = moments_mma_wm(nB);
-  const long long tiles = (long long)((nB + 8 * wm - 1) / (8 * wm)) * moments_mma_groups(L, wm), slots = num_sms();
-  const long long waves = std::max<long long>(1, (NF * tiles + slots * kMmaSlice - 1) / (slots * kMmaSlice));
-  const long long want = std::max<long long>(1, waves * slots / tiles);
-  const long long per = std::max<long long>(4 * kMmaModes, (NF + want - 1) / want);
-  *per_slice = (per + kMmaModes - 1) / kMmaModes * kMmaModes;
-  *nslices = (int)((NF + *per_slice - 1) / *per_slice);
+  const long long tiles = (long long)((nB + 8 * wm - 1) / (8 * wm)) * moments_mma_groups(L, wm);
+  moment_slices(NF, tiles, num_sms(), kMmaModes, kMmaSlice, nslices, per_slice);
 }
 
 // Column tiles per warp: the smallest compiled count that holds the group's columns
