@@ -54,7 +54,8 @@ extern "C" {
 
 /* K_r^{-1} realisations */
 #define FAME_KRINV_EXPLICIT 0 /* exp1/make_explicit_krinv_compact.m */
-#define FAME_KRINV_NESTED 1   /* exp1/make_nested_krinv_instrumented.m */
+#define FAME_KRINV_NESTED 1   /* exp1/make_nested_krinv_instrumented.m; M^{-1} as one product where exact */
+#define FAME_KRINV_NESTED_PCG 2 /* the same with the reference's inner PCG on M always */
 
 /* precision forms of the inner solves */
 #define FAME_PREC_FP64 0  /* plain FP64 throughout */
@@ -208,16 +209,22 @@ FAME_API int fame_yee_lwrq_metrics(fame_ctx* ctx, const void* u1, const void* u2
                                    double h, const double* P, int material_kind, double mp0, double mp1,
                                    double lambda6D, double* metrics, double* slice_z0, double* slice_x0);
 
-/* ---- K_r^{-1} actions ---- */
+/* ---- K_r^{-1} actions ----
+ * FAME_KRINV_NESTED: on the (2N)^6 grid M^{-1} is the same product on 1/eps.  Where that product
+ * inverts M to within tolM (eps positive and finite, 16 ulp * max eps / min eps <= tolM) it takes
+ * the place of the inner PCG: maxitM, prec_mode and tolInner32 then have no effect, every inner
+ * solve counts one iteration (totalMassIterations == massSolveCalls), fp32Iterations and
+ * refineSteps stay 0, and a maxitM that would end the PCG early is no error.  Otherwise, and
+ * always with FAME_KRINV_NESTED_PCG, the inner solves are the PCG that those options describe. */
 typedef struct {
-  int kind;        /* FAME_KRINV_EXPLICIT | FAME_KRINV_NESTED */
+  int kind;        /* FAME_KRINV_EXPLICIT | FAME_KRINV_NESTED | FAME_KRINV_NESTED_PCG */
   int prec_mode;   /* FAME_PREC_FP64 | FAME_PREC_MIXED */
   double tolCG;    /* explicit: Mhat PCG tolerance (1e-10) */
   int maxitCG;     /* explicit: Mhat PCG max iterations (1200) */
   double tolKr;    /* nested: outer K_r PCG tolerance (1e-10) */
-  double tolM;     /* nested: inner M PCG tolerance (1e-12) */
+  double tolM;     /* nested: inner M tolerance (1e-12) */
   int maxitKr;     /* nested (600) */
-  int maxitM;      /* nested (1600) */
+  int maxitM;      /* nested, inner PCG (1600) */
   double epsC;     /* nested preconditioner scale epsC*r./sigma_r (4) */
   int useKrPreconditioner; /* nested (1) */
   double tolInner32; /* mixed: relative tolerance of each FP32 correction solve (3e-6) */
@@ -251,7 +258,7 @@ typedef struct {
   long long maxIterations;
   double maxRelativeResidual;
   long long massSolveCalls;       /* nested: inner M solves */
-  long long totalMassIterations;  /* nested */
+  long long totalMassIterations;  /* nested: their PCG iterations, or one each (see above) */
   long long refineSteps;          /* mixed: FP64 refinement steps */
   long long fp32Iterations;       /* mixed: FP32 PCG iterations */
   long long massApplies;          /* scalar-equivalent mass actions */
@@ -261,9 +268,13 @@ FAME_API int fame_krinv_stats_get(fame_krinv* k, fame_krinv_stats* out);
 FAME_API int fame_krinv_stats_reset(fame_krinv* k);
 
 /* Eigenvector recovery, exp2/recover_original_eigenvectors_exp2.m:12-50:
- * X(:,j) = M^{-1} V Y(:,j) by PCG on diag(M,M,M) (tol, maxit; FAME_PREC_MIXED uses FP64
- * refinement around FP32 PCG), M-normalised; MX = M X.  Y: 2NF x k, X, MX: 3NF x k
- * (device, complex128).  iterations/relres: host arrays of k (may be NULL). */
+ * X(:,j) = M^{-1} V Y(:,j), M-normalised; MX = M X.  Y: 2NF x k, X, MX: 3NF x k (device,
+ * complex128).  iterations/relres: host arrays of k (may be NULL); relres[j] is the true
+ * relative residual ||V y - M x|| / ||V y||.  For N >= 3 a vector whose residual after the
+ * product on 1/eps is within tol reports one iteration, and maxit and prec_mode have no effect
+ * on it.  All others (N <= 2; eps not positive and finite or 16 ulp * max eps / min eps > tol;
+ * a residual above tol; outputs that overlap Y) go through PCG on diag(M,M,M) (tol, maxit;
+ * FAME_PREC_MIXED uses FP64 refinement around FP32 PCG).  maxit < 1 is the PCG's error. */
 FAME_API int fame_recover_eigvecs(fame_basis* b, fame_mass* m, const void* Y, int k, double tol,
                                   int maxit, int prec_mode, void* X, void* MX, int* iterations,
                                   double* relres);

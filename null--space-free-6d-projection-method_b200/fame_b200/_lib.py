@@ -23,7 +23,7 @@ FAME_ERR_BREAKDOWN = 9
 
 FAME_F64, FAME_F32 = 0, 1
 FAME_MASS_SCALAR, FAME_MASS_FULL3, FAME_MASS_COL3, FAME_MASS_COLS12 = 0, 1, 2, 3
-FAME_KRINV_EXPLICIT, FAME_KRINV_NESTED = 0, 1
+FAME_KRINV_EXPLICIT, FAME_KRINV_NESTED, FAME_KRINV_NESTED_PCG = 0, 1, 2
 FAME_PREC_FP64, FAME_PREC_MIXED = 0, 1
 
 

@@ -434,9 +434,14 @@ def make_explicit_krinv_compact(sys: QSystem, tolCG=1e-10, maxitCG=1200, precisi
 
 
 def make_nested_krinv_instrumented(sys: QSystem, epsC=4.0, tolKr=1e-10, tolM=1e-12, maxitKr=600,
-                                   maxitM=1600, useKrPreconditioner=True, precision="fp64", **kw):
-    """exp1/make_nested_krinv_instrumented.m:1-174 — returns ``(KrInvOp, getStats)``."""
-    o = _opts(kind=L.FAME_KRINV_NESTED, tolKr=tolKr, tolM=tolM, maxitKr=maxitKr, maxitM=maxitM,
+                                   maxitM=1600, useKrPreconditioner=True, precision="fp64", inner_pcg=False, **kw):
+    """exp1/make_nested_krinv_instrumented.m:1-174 — returns ``(KrInvOp, getStats)``.
+
+    Where the material allows it to within ``tolM``, M^{-1} is one product on 1/eps instead of an
+    inner PCG: ``maxitM`` and ``precision`` then have no effect and each inner solve counts one
+    iteration.  ``inner_pcg=True`` keeps the reference's inner PCG (and its counts) always.
+    """
+    o = _opts(kind=L.FAME_KRINV_NESTED_PCG if inner_pcg else L.FAME_KRINV_NESTED, tolKr=tolKr, tolM=tolM, maxitKr=maxitKr, maxitM=maxitM,
               epsC=float(epsC), useKrPreconditioner=int(bool(useKrPreconditioner)),
               prec_mode=L.FAME_PREC_MIXED if precision == "mixed" else L.FAME_PREC_FP64, **kw)
     op = KrInv(sys, o)

@@ -20,7 +20,9 @@ __all__ = ["compute_yee_lwrq_metrics", "reconstruct_fields_direct_grid", "recove
 def recover_original_eigenvectors(Y, sys: QSystem, tol=1e-12, maxit=3000, precision="fp64"):
     """exp2/recover_original_eigenvectors_exp2.m:12-57 — X = M^{-1} V Y, M-normalised.
 
-    Returns ``(X, MX, info)`` with X, MX of shape (3NF, k) (column-major views).
+    Returns ``(X, MX, info)`` with X, MX of shape (3NF, k) (column-major views).  From N = 3 on,
+    M^{-1} is one product on 1/eps where that reaches ``tol`` (one iteration is reported, and
+    ``maxit`` and ``precision`` have no effect); otherwise the reference's PCG runs.
     """
     Yc = Y.t().contiguous() if Y.dim() == 2 else Y.reshape(1, -1).contiguous()
     k = Yc.shape[0]
