@@ -208,6 +208,10 @@ FAME_API int fame_apply_Mhat_C_scalar_compact_noalloc(fame_basis* b, fame_mass* 
 FAME_API int fame_yee_lwrq_metrics(fame_ctx* ctx, const void* u1, const void* u2, const void* u3, int n,
                                    double h, const double* P, int material_kind, double mp0, double mp1,
                                    double lambda6D, double* metrics, double* slice_z0, double* slice_x0);
+/* The same with the slices row-major (C arrays: slice_z0[x][y], slice_x0[y][z]). */
+FAME_API int fame_yee_lwrq_metrics_rows(fame_ctx* ctx, const void* u1, const void* u2, const void* u3, int n,
+                                        double h, const double* P, int material_kind, double mp0, double mp1,
+                                        double lambda6D, double* metrics, double* slice_z0, double* slice_x0);
 
 /* ---- K_r^{-1} actions ----
  * FAME_KRINV_NESTED: on the (2N)^6 grid M^{-1} is the same product on 1/eps.  Where that product

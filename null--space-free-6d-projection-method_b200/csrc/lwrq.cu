@@ -296,11 +296,12 @@ __global__ void __launch_bounds__(256) k_lwrq_xy(const double* __restrict__ inA,
 // statistics of E and M with rho = E/M and l0 = sum a / sum b (out1, k_lwrq_ab): out [0] sum E,
 // [1] sum M, [2] non-finite count, [3] sum M (rho - l0)^2, [4] sum M (rho - l0), [5] min M,
 // [6] max M.  The window keeps the sums of a and b to rounding, so l0 is lambda3D to rounding
-// and the sums about it lose nothing when the host moves them to lambda3D.
+// and the sums about it lose nothing when the host moves them to lambda3D.  s0, s1: strides of
+// the slices' two indices.
 constexpr int kZRun = 24, kZStep = 4;
 __global__ void __launch_bounds__(256) k_lwrq_z(const double* __restrict__ inA, const double* __restrict__ inB, int q,
-                                                Window w, const double* __restrict__ out1, double* z0, double* x0,
-                                                double* out, double* partials, unsigned* counter) {
+                                                Window w, const double* __restrict__ out1, double* z0, double* x0, int s0,
+                                                int s1, double* out, double* partials, unsigned* counter) {
   constexpr int R = kLwrqR, T = 2 * R + 1;
   __shared__ double red[8][7];
   __shared__ bool am_last;
@@ -337,8 +338,8 @@ __global__ void __launch_bounds__(256) k_lwrq_z(const double* __restrict__ inA, 
           v[4] += M * dv;
           v[5] = fmin(v[5], M);
           v[6] = fmax(v[6], M);
-          if (z0 && k + u == c) z0[col] = rho;
-          if (x0 && i == c) x0[j + (long long)q * (k + u)] = rho;
+          if (z0 && k + u == c) z0[i * s0 + j * s1] = rho;
+          if (x0 && i == c) x0[j * s0 + (k + u) * s1] = rho;
         }
       }
 #pragma unroll
@@ -424,9 +425,10 @@ __global__ void __launch_bounds__(256) k_lwrq_resid(YeeGeom g, YeeMat mt, YeeTab
 
 using namespace fame;
 
-extern "C" int fame_yee_lwrq_metrics(fame_ctx* ctx, const void* u1, const void* u2, const void* u3, int n, double h,
-                                     const double* P, int material_kind, double mp0, double mp1, double lambda6D,
-                                     double* metrics, double* slice_z0, double* slice_x0) {
+// rows: the slices row-major, the first index slowest (column-major otherwise)
+static int lwrq_metrics(fame_ctx* ctx, const void* u1, const void* u2, const void* u3, int n, double h,
+                        const double* P, int material_kind, double mp0, double mp1, double lambda6D, double* metrics,
+                        double* slice_z0, double* slice_x0, bool rows) {
   if (!ctx || !u1 || !u2 || !u3 || !P || !metrics || n < 1 || !(h > 0.0) || (material_kind != 0 && material_kind != 1))
     return fail(FAME_ERR_INVALID, "fame_yee_lwrq_metrics arguments");
   if (!(std::fabs(lambda6D) > 0.0)) return fail(FAME_ERR_INVALID, "lambda6D must be nonzero");
@@ -484,7 +486,8 @@ extern "C" int fame_yee_lwrq_metrics(fame_ctx* ctx, const void* u1, const void* 
   if (separable) k_lwrq_ab<true><<<gab, kAbTile * kAbTile, 0, s>>>(g, mt, tb, lambda6D, a, b, sc, part, counter);
   else k_lwrq_ab<false><<<gab, kAbTile * kAbTile, 0, s>>>(g, mt, tb, lambda6D, a, b, sc, part, counter);
   k_lwrq_xy<<<gxy, 256, 0, s>>>(a, b, T, U, q, w);
-  k_lwrq_z<<<gz, 256, 0, s>>>(T, U, q, w, sc, slice_z0 ? z0 : nullptr, slice_x0 ? x0 : nullptr, sc + 6, part, counter);
+  k_lwrq_z<<<gz, 256, 0, s>>>(T, U, q, w, sc, slice_z0 ? z0 : nullptr, slice_x0 ? x0 : nullptr, rows ? q : 1,
+                             rows ? 1 : q, sc + 6, part, counter);
   ::fame::count_launch(4);
   if (slice_z0 || slice_x0) {
     k_lwrq_dev<<<(q * q + 255) / 256, 256, 0, s>>>(slice_z0 ? z0 : nullptr, slice_x0 ? x0 : nullptr, q * q, sc + 6);
@@ -537,3 +540,19 @@ extern "C" int fame_yee_lwrq_metrics(fame_ctx* ctx, const void* u1, const void* 
   if (slice_z0 || slice_x0) FAME_CUDA_TRY(cudaStreamSynchronize(s));
   return FAME_OK;
 }
+
+extern "C" {
+
+int fame_yee_lwrq_metrics(fame_ctx* ctx, const void* u1, const void* u2, const void* u3, int n, double h,
+                          const double* P, int material_kind, double mp0, double mp1, double lambda6D, double* metrics,
+                          double* slice_z0, double* slice_x0) {
+  return lwrq_metrics(ctx, u1, u2, u3, n, h, P, material_kind, mp0, mp1, lambda6D, metrics, slice_z0, slice_x0, false);
+}
+
+int fame_yee_lwrq_metrics_rows(fame_ctx* ctx, const void* u1, const void* u2, const void* u3, int n, double h,
+                               const double* P, int material_kind, double mp0, double mp1, double lambda6D,
+                               double* metrics, double* slice_z0, double* slice_x0) {
+  return lwrq_metrics(ctx, u1, u2, u3, n, h, P, material_kind, mp0, mp1, lambda6D, metrics, slice_z0, slice_x0, true);
+}
+
+}  // extern "C"

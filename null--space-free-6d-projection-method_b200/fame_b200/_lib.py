@@ -121,6 +121,7 @@ SIGNATURES = {
     "fame_mass_adjoint": [P, P, I, P, I, C.POINTER(D)],
     "fame_mass_adjoint_fields": [P, P, I, C.POINTER(P), I, C.POINTER(D)],
     "fame_yee_lwrq_metrics": [P, P, P, P, I, D, C.POINTER(D), I, D, D, D, C.POINTER(D), C.POINTER(D), C.POINTER(D)],
+    "fame_yee_lwrq_metrics_rows": [P, P, P, P, I, D, C.POINTER(D), I, D, D, D, C.POINTER(D), C.POINTER(D), C.POINTER(D)],
     "fame_solve_batch": [I, I, C.POINTER(I), C.POINTER(P), C.POINTER(D), C.POINTER(D),
                          C.POINTER(fame_krinv_opts), I, D, I, I, C.c_ulonglong, C.POINTER(D),
                          C.POINTER(fame_lanczos_info), C.POINTER(I)],

@@ -240,13 +240,14 @@ def compute_yee_lwrq_metrics(fields, lambda6D, P, n, h, material=("exp", 4.0, 1.
     mp1 = float(material[2]) if len(material) > 2 else 0.0
     out = (C.c_double * 10)()
     q = 2 * n + 1
-    z0, x0 = (np.empty((q, q), order="F") if save_spatial else None for _ in range(2))
+    z0, x0 = (np.empty((q, q)) if save_spatial else None for _ in range(2))
     dp = C.POINTER(C.c_double)
-    call("fame_yee_lwrq_metrics", ctx.bind(), _ptr(us[0]), _ptr(us[1]), _ptr(us[2]), int(n), float(h), Pc, kind,
+    call("fame_yee_lwrq_metrics_rows", ctx.bind(), _ptr(us[0]), _ptr(us[1]), _ptr(us[2]), int(n), float(h), Pc, kind,
          mp0, mp1, float(lambda6D), out, *(a.ctypes.data_as(dp) if a is not None else None for a in (z0, x0)))
     met = dict(h=h, n=n, halfWidth=n * h, lambda6D=lambda6D)
     met.update({k: float(out[i]) for i, k in enumerate(LWRQ_KEYS)})
     spatial = None
     if save_spatial:
-        spatial = dict(relativeDeviation_z0=z0, relativeDeviation_x0=x0, coord=np.arange(-n, n + 1) * h, lambda3D=met["lambda3D"], lambda6D=lambda6D, h=h, n=n)
+        spatial = dict(relativeDeviation_z0=z0, relativeDeviation_x0=x0, coord=np.arange(-n, n + 1) * h,
+                       lambda3D=met["lambda3D"], lambda6D=lambda6D, h=h, n=n)
     return met, spatial

@@ -78,3 +78,30 @@ def test_lwrq_refusals(cuda_device):
     with pytest.raises(F.FameError) as e:
         F.compute_yee_lwrq_metrics(bad, 0.05, F.configs.P_GOLDEN, n, 0.05, ("cos", 12.0))
     assert e.value.status == F._lib.FAME_ERR_INVALID
+
+
+@pytest.mark.parametrize("n", [1, 4, 9, 20])
+def test_slices_in_both_layouts(cuda_device, n):
+    """Python hands the slices out as C-contiguous arrays; the C entry's column-major slices hold
+    the same values."""
+    import ctypes as C
+    import torch
+    import fame_b200 as F
+    from fame_b200 import _lib as L
+    m, q = 2 * n + 3, 2 * n + 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    us = [torch.complex(torch.randn(m ** 3, dtype=torch.float64, device="cuda", generator=g),
+                        torch.randn(m ** 3, dtype=torch.float64, device="cuda", generator=g)) for _ in range(3)]
+    P = np.asarray(F.configs.P_GOLDEN, dtype=np.float64)
+    _, sp = F.compute_yee_lwrq_metrics(us, 0.05, P, n, 0.0125, ("cos", 12.0), save_spatial=True)
+    cols = [np.empty((q, q), order="F") for _ in range(2)]
+    ctx = F.core.default_context()
+    out = (C.c_double * 10)()
+    dp = C.POINTER(C.c_double)
+    F._lib.call("fame_yee_lwrq_metrics", ctx.bind(), *[C.c_void_p(u.data_ptr()) for u in us], n, 0.0125,
+                (C.c_double * 18)(*P.reshape(6, 3).ravel(order="F")), 1, 12.0, 0.0, 0.05, out,
+                *[a.ctypes.data_as(dp) for a in cols])
+    for a, key in zip(cols, ("relativeDeviation_z0", "relativeDeviation_x0")):
+        assert sp[key].flags.c_contiguous and sp[key].shape == (q, q)
+        assert np.array_equal(sp[key], a)
