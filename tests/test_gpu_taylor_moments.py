@@ -71,3 +71,39 @@ def test_phase_reduction_at_large_arguments(cuda_device):
                                 torch.arange(16, device=cuda_device, dtype=torch.int64)))
         ref = (1 + 0.5j) * np.exp(1j * v * R[:, 0])
         assert np.max(np.abs(u.cpu().numpy() - ref)) < 1e-12
+
+
+def test_phase_accuracy_around_multiples_of_half_pi(cuda_device):
+    """e^{ix} at and within a few ulp of multiples of pi/2 and of the octant boundaries between them,
+    up to and past the end of the reduction (2^19 pi/2), against 80-bit sin and cos: absolute error
+    below 3e-16 (half an ulp each of the reduced argument, of the result and of the polynomials'
+    last products, 5.6e-17 at most).  One point per block makes the block's center the point, and
+    at order 0 the field is the phase."""
+    import torch
+    import fame_b200 as F
+    if np.finfo(np.longdouble).nmant < 63:
+        pytest.skip("no 80-bit reference")
+    rng = np.random.default_rng(9)
+    k = np.unique(np.concatenate([np.arange(300), 2 ** np.arange(0, 20), rng.integers(1, 2 ** 19, 900),
+                                  2 ** 19 - np.arange(12)]))
+    half_pi = (np.longdouble(np.pi) + np.longdouble(1.2246467991473532e-16)) / 2
+    x = np.concatenate([k * half_pi, (k + 0.5) * half_pi]).astype(np.float64)
+    x = np.concatenate([x, np.nextafter(x, np.inf), np.nextafter(x, -np.inf), x * (1 + 3 * 2.0 ** -52),
+                        rng.uniform(-40, 40, 2000), [823549.0, np.nextafter(823549.0, 0), 1e6, 1e300]])
+    x = np.concatenate([x, -x])
+    assert x.size < 65536
+    M = x.size
+    R = np.zeros((3, M))
+    R[0] = x
+    Q = np.zeros((3, 2))
+    Q[0] = 1.0
+    u = F.taylor_on_blocks(torch.tensor([1.0, 0.0], device=cuda_device, dtype=torch.complex128),
+                           torch.as_tensor(Q, device=cuda_device).t(), torch.as_tensor(R, device=cuda_device).t(), 0,
+                           (torch.arange(M + 1, device=cuda_device, dtype=torch.int64),
+                            torch.arange(M, device=cuda_device, dtype=torch.int64))).cpu().numpy()
+    xl = x.astype(np.longdouble)
+    small = np.abs(x) < 2.0 ** 60  # the 80-bit functions reduce arguments up to 2^63
+    err = np.maximum(np.abs(u.real - np.cos(xl)), np.abs(u.imag - np.sin(xl)))[small]
+    assert float(err.max()) < 3e-16
+    ref = np.stack([np.cos(x), np.sin(x)])[:, ~small]
+    assert np.max(np.abs(np.stack([u.real, u.imag])[:, ~small] - ref)) < 3e-16
