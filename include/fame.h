@@ -240,9 +240,11 @@ typedef struct {
                              material 1/eps, C^{-1} B^H (I3 (x) M^{-1}) B C^{-1}; the stopping
                              test stays ||b - Mhat u|| <= tolCG ||b|| (1).  0: plain CG as the
                              reference's pcg(Mhat, ...) in exp1/make_explicit_krinv_compact.m:43 */
-  int passColumns; /* columns per CTA of the inner solves' pass A/C kernels: 0 = built-in default;
-                      alternatives 2, 4 (2N = 10), 2, 4 (2N = 8), 4, 6 (2N = 6); other values
-                      fall back to the default (fame_b200.autotune picks it per problem) */
+  int passColumns; /* kernels of the inner solves' passes A and C: 0 = built-in default (at
+                      2N <= 8 the three fields side by side, one column of the grid per CTA);
+                      alternatives with that many columns per CTA and the fields one after
+                      another: 2, 4 (2N = 10), 2, 4 (2N = 8), 4, 6 (2N = 6); other values fall
+                      back to the default (fame_b200.autotune picks it per problem) */
   double refineTarget; /* explicit, mixed: the FP64 refinement of each Mhat solve stops once
                           ||bhat - Mhat u|| <= refineTarget * tolCG * ||bhat||, in (0, 1] (0.1).
                           1 is the stopping rule of the reference's pcg (relres <= tolCG); the

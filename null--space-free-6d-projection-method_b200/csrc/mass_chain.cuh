@@ -92,10 +92,11 @@ int run_chain(int n, const Pro& pro, const Epi& epi, C<T>* work, const TE* Et, l
 
 // Columns per CTA of the linear-field passes (one line per thread).
 // n >= 10: one column (100 lines and more) per CTA, several CTAs per SM (measured 1-3 % faster
-// K_r^{-1} actions than two columns, in both precision forms).  Below, two: n^3 / 2 CTAs reach
-// more SMs than the 512-thread CTAs that eight to sixteen columns would make (18 at n = 6), and
-// fill whole warps better than single columns.  Ten eigenpairs in FP64: N=2 24.8 -> 21.9 ms,
-// N=3 35.6 -> 26.3 ms, N=4 53.7 -> 44.7 ms (one column: 21.8 / 27.5 / 46.7 ms).
+// K_r^{-1} actions than two columns, in both precision forms).  Below, two, which only the
+// one-field products still use (chain_par takes the others, one column per CTA): n^3 / 2 CTAs
+// reach more SMs than the 512-thread CTAs that eight to sixteen columns make, and fill whole
+// warps better than single columns.  FP64 products of 24 vectors, two / one / eight and more
+// columns: N=3 35.3 / 38.8 / 36.3 us, N=4 154.5 / 175 / 168 us; single vectors within 2 us.
 template <int n, typename T> struct LinCols {
   static constexpr int value = n >= 10 ? 1 : 2;
   static_assert((n * n * n) % value == 0 && value * n * n <= 512, "linear chain tiling");
@@ -139,10 +140,14 @@ int chain_par(const Pro& pro, const Epi& epi, C<T>* work, const TE* Et, long lon
   return FAME_OK;
 }
 
-// Columns per CTA of the linear passes: LinCols by default; `cols` selects one of the
-// alternatives compiled for the Bloch-path sizes (n = 6, 8, 10), any other value the default.
-// The choice changes the CTA grouping (and so the order of the grid reductions), not the
-// arithmetic of a mode.
+// The linear chain of n: several fields side by side at n <= 8 (k_passA_par, one column per CTA),
+// one after another with LinCols columns per CTA above and for one field.  `cols` selects one of
+// the alternatives compiled for the Bloch-path sizes (n = 6, 8, 10): that many columns per CTA
+// and, at n <= 8 too, the fields one after another; any other value is the default.  The choice
+// changes the kernels and the order of the grid reductions, not the arithmetic of a mode.  Where
+// many instances share the GPU the larger CTAs can win: eight concurrent solves at N=4 take 294
+// against 312 ms (FP64) and 218 against 225 ms (mixed) with two columns; a solve alone, and
+// batches at N=3 and N=5, are fastest with the default.
 template <int n, typename T, int F, class Pro, class Epi, typename TE>
 int chain_lin_n(const Pro& pro, const Epi& epi, C<T>* work, const TE* Et, long long NF, cudaStream_t st, Gate gate,
                 int cols) {

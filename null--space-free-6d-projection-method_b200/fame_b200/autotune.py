@@ -4,9 +4,11 @@ Three options of the K_r^{-1} operator decide how its work reaches the GPU but n
 what a mode computes: ``checkEvery`` (PCG iterations queued behind the device's
 active flag between two host reads of the PCG state), ``useGraphs`` (replay the
 iteration bodies from captured CUDA graphs or launch them one by one) and
-``passColumns`` (columns of the 6D grid per CTA in the pass A/C kernels of the
-inner solves; alternatives are compiled for 2N = 6, 8, 10, the sizes of the
-Bloch-path workload).  The best combination depends on the problem size (small N is
+``passColumns`` (the pass A/C kernels of the inner solves: by default the three
+fields side by side with one column of the 6D grid per CTA at 2N <= 8, else one
+after another; the alternatives, compiled for 2N = 6, 8, 10, the sizes of the
+Bloch-path workload, take that many columns per CTA with the fields one after
+another).  The best combination depends on the problem size (small N is
 launch-bound, large N is not) and on the host, so it is measured: each candidate
 times a few K_r^{-1} actions on a fixed vector after a warm-up, and the fastest
 wins.  Candidates that differ only in the schedule must give bitwise-identical
