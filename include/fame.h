@@ -110,7 +110,9 @@ FAME_API int fame_selftest_bounded_wait(fame_mass* m, unsigned poll_limit);
 /* The same expiry in one kernel, without the report: kernel 0 = pass B (FP32), 1 = pass B of the
  * mass adjoint, 2 = the Gram-Schmidt tile kernel.  The fault word stays set for the next call
  * that checks it: fame_ctx_sync, fame_mass_adjoint(_fields), fame_lanczos, fame_osi_eigs,
- * fame_rayleigh_ritz and the batched solves then fail with FAME_ERR_CUDA. */
+ * fame_rayleigh_ritz and the batched solves then fail with FAME_ERR_CUDA.  The word belongs to
+ * the device: fame_ctx_sync of every context that was there reports it once, whichever call
+ * cleared it; the other calls report what gave up while they ran, or was not reported yet. */
 FAME_API int fame_selftest_expired_wait(fame_mass* m, int kernel, unsigned poll_limit);
 
 /* Replaces applyMij_rank1_exact(x,kernelFFT,plan) — exp1/applyMij_rank1_exact.m:1-6

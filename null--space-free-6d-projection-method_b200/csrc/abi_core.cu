@@ -167,7 +167,10 @@ int num_sms() {
   return v > 0 ? v : 148;
 }
 
-int check_fault(fame_ctx* ctx) {
+// Whether a bounded wait of ctx's device has given up since the fault word was last cleared
+// (synchronises ctx's stream); counts and clears it.
+static int take_fault(fame_ctx* ctx, bool* set) {
+  *set = false;
   unsigned* p = g_fault[ctx->device].load();
   if (!p) return FAME_OK;
   FAME_CUDA_TRY(cudaMemcpyAsync(ctx->pinned, p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
@@ -175,18 +178,26 @@ int check_fault(fame_ctx* ctx) {
   unsigned v = 0;
   std::memcpy(&v, ctx->pinned, sizeof(unsigned));
   if (v == 0) return FAME_OK;
-  g_faults_seen[ctx->device].fetch_add(1);  // before the word is cleared: see FaultWatch
+  *set = true;
+  g_faults_seen[ctx->device].fetch_add(1);  // before the word is cleared, for the other contexts
   FAME_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(unsigned), ctx->stream));
+  return FAME_OK;
+}
+
+static int fault_since(fame_ctx* ctx, unsigned seen) {
+  bool set = false;
+  FAME_TRY(take_fault(ctx, &set));
+  const unsigned now = g_faults_seen[ctx->device].load();
+  if (!set && now == seen) return FAME_OK;
+  ctx->faults_seen = now;
   return fail(FAME_ERR_CUDA, "a bounded device-side wait gave up (bulk copy never completed); results are invalid");
 }
 
+int check_fault(fame_ctx* ctx) { return fault_since(ctx, ctx->faults_seen); }
+
 FaultWatch::FaultWatch(fame_ctx* c) : ctx(c), seen(g_faults_seen[c->device].load()) {}
 
-int FaultWatch::check() {
-  FAME_TRY(check_fault(ctx));
-  if (g_faults_seen[ctx->device].load() == seen) return FAME_OK;
-  return fail(FAME_ERR_CUDA, "a bounded device-side wait gave up during this call; results are invalid");
-}
+int FaultWatch::check() { return fault_since(ctx, seen); }
 
 int ctx_workspace(fame_ctx* ctx, size_t bytes, void** out) {
   if (bytes > ctx->ws_bytes) {
@@ -287,6 +298,7 @@ int fame_ctx_create(int device, fame_ctx** out) {
     return fail(FAME_ERR_CUDA, "context resources");
   }
   c->stream = c->own;
+  c->faults_seen = g_faults_seen[device].load();
   *out = c;
   return FAME_OK;
 }

@@ -13,6 +13,7 @@ struct fame_ctx {
   void* ws = nullptr;      // grow-only device workspace (ctx_workspace)
   size_t ws_bytes = 0;
   std::vector<void*> allocs;
+  unsigned faults_seen = 0;  // count of the device's reported faults at this context's last check
 };
 
 namespace fame {
@@ -75,11 +76,12 @@ struct StreamOrderedAlloc {
 };
 // copy a small device struct to host (synchronises the stream)
 int read_back(fame_ctx* ctx, const void* dsrc, void* hdst, size_t bytes);
-// FAME_ERR_CUDA (and clears the word) if a bounded device-side wait gave up on ctx's device
+// FAME_ERR_CUDA if a bounded device-side wait gave up on ctx's device since the context's last
+// check (or creation), also where another context's check found the device's fault word first
+// and cleared it: the word does not say whose work was spoiled, so every context hears of it
+// once.  Synchronises ctx's stream and clears the word.
 int check_fault(fame_ctx* ctx);
-// For a call whose own result rests on bounded waits: check() synchronises ctx's stream and
-// fails if any wait of the device gave up since the construction, also where another host
-// thread's check found the device's fault word first and cleared it.
+// The same for one call whose own result rests on bounded waits: since the construction.
 class FaultWatch {
   fame_ctx* ctx;
   unsigned seen;

@@ -336,6 +336,7 @@ extern "C" int fame_rayleigh_ritz(fame_basis* b, fame_mass* m, void* Y, int k, d
   double* lamd = c2.take<double>(k);
   double* resd = c2.take<double>((size_t)kGramBlocksMax * 2 * k);
   double2* Yd = (double2*)Y;
+  FaultWatch watch(ctx);
   // Z = K_r Y = V^* M^{-1} V Y, one chain per column on the material 1/eps
   for (int j = 0; j < k; ++j) {
     ProVy pro;
@@ -352,7 +353,7 @@ extern "C" int fame_rayleigh_ritz(fame_basis* b, fame_mass* m, void* Y, int k, d
   FAME_CUDA_TRY(cudaGetLastError());
   std::vector<double2> hg(npair);
   FAME_TRY(copy_to_host(ctx, gram, hg.data(), npair * sizeof(double2)));
-  FAME_TRY(check_fault(ctx));
+  FAME_TRY(watch.check());
   std::vector<cd> G((size_t)k * k), B((size_t)k * k);
   for (int p = 0; p < k * k; ++p) {
     G[p] = cd(hg[p].x, hg[p].y);

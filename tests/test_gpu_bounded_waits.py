@@ -58,3 +58,43 @@ def test_selftest_refuses_other_arguments(cuda_device):
     m = _mass(1)
     for kernel, limit in ((3, 16), (-1, 16), (0, 0), (1, 1 << 21)):
         assert L.lib.fame_selftest_expired_wait(m.h, kernel, limit) == L.FAME_ERR_INVALID
+
+
+def test_every_context_hears_of_a_fault_once(cuda_device):
+    """The fault word is the device's: the context whose check clears it need not be the one whose
+    work was spoiled, so the others report it at their next synchronisation too, once; a context
+    made afterwards does not, and calls that check their own run are not refused for it."""
+    import torch
+    import fame_b200 as F
+    m = _mass(2)
+    m.ctx.sync()
+    other, third = F.Context(0), F.Context(0)
+    _expire(m, PASS_B)
+    for ctx in (other, m.ctx):  # the first of them clears the word
+        with pytest.raises(F.FameError) as e:
+            ctx.sync()
+        assert e.value.status == F._lib.FAME_ERR_CUDA
+        ctx.sync()
+    late = F.Context(0)
+    late.sync()
+    # a healthy call of a context that has not synchronised since is not refused
+    m3 = F.MassBackend(torch.as_tensor(O.material_separable_cos(2, 12.0), device="cuda"), 2, ctx=third)
+    X = torch.as_tensor(O.start_vector(3, 3 * m.NF), device="cuda").reshape(-1, 1)
+    g = [torch.ones(m.NF, dtype=torch.float64, device="cuda")]
+    assert np.array_equal(F.grad.mass_adjoint(m3, X, g), F.grad.mass_adjoint(m, X, g))
+    with pytest.raises(F.FameError):
+        third.sync()
+    third.sync()
+
+
+def test_rayleigh_ritz_reports_an_expired_wait(cuda_device):
+    import torch
+    import fame_b200 as F
+    m = _mass(2)
+    sysq = F.build_q_system(m, F.configs.P_GOLDEN, F.configs.Q_PHYS)
+    Y = torch.stack([F.start_vector(s, sysq.nr) for s in (1, 2, 3)], 0).t()
+    _expire(m, PASS_B)
+    with pytest.raises(F.FameError) as e:
+        F.rayleigh_ritz(sysq, Y)
+    assert e.value.status == F._lib.FAME_ERR_CUDA
+    assert F.rayleigh_ritz(sysq, Y)[0].shape == (3,)
