@@ -30,6 +30,8 @@ struct fame_mass {
   double* EtInv64 = nullptr;  // NF^-1 / E in the same tile order: the inverse mass operator
   float* EtInv32 = nullptr;
   fame::MaterialRange* range = nullptr;  // device: smallest and largest E, whether all E are positive and finite
+  unsigned long long rangeWords[3] = {0, 0, 0};  // the same on the host once rangeRead (read_range)
+  bool rangeRead = false;
   void* store = nullptr;                 // the one allocation behind the pointers above
   cudaEvent_t ready = nullptr;           // recorded behind the tables and range above
 };
@@ -100,7 +102,8 @@ int ctx_workspace(fame_ctx* ctx, size_t bytes, void** out);
 // and finite, and the chain's rounding (a few ulp of the largest field value, amplified by
 // max E / min E when the residual is taken) below tol.  r: the handle's range, read back.
 bool exact_inverse_ok(const MaterialRange& r, double tol);
-// the handle's range on the host, read on ctx's stream behind the handle's set-up
+// the handle's range on the host, with ctx's stream ordered behind the handle's set-up; the first
+// call for a handle reads it from the device (the tables it describes never change)
 int read_range(fame_ctx* ctx, fame_mass* m, MaterialRange* r);
 // Taylor block moments on the tensor cores (taylor_tc.cu): launch shape and the
 // FP32 partial-moment buffer (out_floats) it needs.

@@ -238,8 +238,12 @@ bool exact_inverse_ok(const MaterialRange& r, double tol) {
 }
 
 int read_range(fame_ctx* ctx, fame_mass* m, MaterialRange* r) {
+  static_assert(sizeof(*r) == sizeof(m->rangeWords), "host copy of the range");
   FAME_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, m->ready, 0));
-  return read_back(ctx, m->range, r, sizeof(*r));
+  if (!m->rangeRead) FAME_TRY(read_back(ctx, m->range, m->rangeWords, sizeof(m->rangeWords)));
+  m->rangeRead = true;
+  std::memcpy(r, m->rangeWords, sizeof(*r));
+  return FAME_OK;
 }
 
 }  // namespace fame
