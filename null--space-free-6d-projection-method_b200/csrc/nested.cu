@@ -293,8 +293,10 @@ __global__ void k_exact_init(const double2* b, double2* x, double2* r, const dou
     st->pend = 0;
     st->active = t.v[0] > 0.0 && isfinite(t.v[0]) && maxit > 0 ? 1 : 0;
     if (st->active && !(t.v[1] > 0.0 && isfinite(t.v[1]))) {
+      // breakdown; a negative scale still takes the one step of the inner-PCG form, which is
+      // exact where K_r M1 is a multiple of the identity
       st->pad = 4;
-      st->active = 0;
+      if (!(t.v[1] < 0.0 && isfinite(t.v[1]))) st->active = 0;
     }
   });
 }
@@ -405,7 +407,7 @@ struct EpiOuterVH {
     st->rho = rho;
     st->beta = rho / st->rho1;
     st->iter += 1;
-    if (!isfinite(rr) || !isfinite(rho)) {
+    if (st->pad == 4 || !isfinite(rr) || !isfinite(rho)) {
       st->pad = 4;
       st->active = 0;
     } else if (rr <= kRecheck * t.v[2] || rho <= kRecheck * t.v[6]) {
@@ -534,12 +536,13 @@ static int exact_outer_solve(fame_krinv* K, const double2* b, double2* x, OuterS
     if (!std::isfinite(h.bnorm2)) return fail(FAME_ERR_NONFINITE, "Nested K_r^{-1} input contains NaN/Inf");
     chunk = every;
     if (h.active) continue;
-    if (h.pad == 4) {
+    if (h.pad == 4 && !h.pend) {
       *flag = 4;
       break;
     }
+    const bool broken = h.pad == 4;
     const bool recheck = h.pad == 8;
-    if (!recheck && !(h.rr <= h.tolb2)) break;  // iteration limit
+    if (!broken && !recheck && !(h.rr <= h.tolb2)) break;  // iteration limit
     if (h.bnorm2 == 0.0) {
       *flag = 0;
       break;
@@ -552,6 +555,10 @@ static int exact_outer_solve(fame_krinv* K, const double2* b, double2* x, OuterS
     FAME_TRY((run_chain<double, 3>(K->n, pro, epi, K->b64.work, K->m->EtInv64, NF, s)));
     ++products;
     FAME_TRY(read_back(K->ctx, K->ost, &h, sizeof(OuterState)));
+    if (broken) {  // the residual it broke down with decides
+      *flag = 4;
+      break;
+    }
     if (h.rr <= h.tolb2 || (!recheck && !K->o.verifyTrueResidual)) {
       *flag = 0;
       break;

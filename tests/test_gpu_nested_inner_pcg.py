@@ -62,3 +62,27 @@ def test_unknown_kinds_stay_refused(cuda_device):
         with pytest.raises(F.FameError) as e:
             F.KrInv(sg, o)
         assert e.value.status == F._lib.FAME_ERR_INVALID
+
+
+@pytest.mark.parametrize("N", [1, 2, 3])
+@pytest.mark.parametrize("inner_pcg", [False, True])
+def test_negative_preconditioner_scale(cuda_device, N, inner_pcg):
+    """epsC < 0 breaks the outer PCG down after one step, in both inner forms: that step is the
+    solution on eps = 1, where K_r is |q|^2 (accepted on its residual), and the breakdown's error on
+    any other material."""
+    import torch
+    import fame_b200 as F
+    b = None
+    for E, ok in ((np.ones((2 * N) ** 6), True), (O.material_separable_cos(N, 12.0), False)):
+        sg = F.build_q_system(F.MassBackend(torch.as_tensor(E, device=cuda_device), N), F.configs.P_GOLDEN,
+                              F.configs.Q_PHYS)
+        b = torch.as_tensor(O.start_vector(5, sg.nr), device=cuda_device)
+        op, _ = F.make_nested_krinv_instrumented(sg, epsC=-1.0, inner_pcg=inner_pcg)
+        if ok:
+            y = op(b)
+            ref = b / sg.sigmaR
+            assert float(torch.linalg.norm(y - ref) / torch.linalg.norm(ref)) < 1e-9
+        else:
+            with pytest.raises(F.FameError) as e:
+                op(b)
+            assert e.value.status == F._lib.FAME_ERR_NOT_CONVERGED
